@@ -2537,10 +2537,18 @@ static int last_step_streamed(nmg_ctx *c, double t, double dt, double *host_u,
     }
     CK(cudaEventRecord(c->fork_ev, c->stream));
     CK(cudaStreamWaitEvent(c->stream2, c->fork_ev, 0));
+    // "fvc" passes flux differences from its first kernel to its second through the
+    // scratch, so each of the two streams has its own half of it
+    const int half = c->fvdiv_cap / 2;
+    const bool two = !c->mixed && (!c->fv || half > 0);
     int k = 0;
     for (int64_t ea = 0; ea < E; ea += chunk, k++) {
       const int64_t eb = std::min(E, ea + chunk);
-      cudaStream_t sk = ((k & 1) && !c->mixed) ? c->stream2 : c->stream;
+      cudaStream_t sk = ((k & 1) && two) ? c->stream2 : c->stream;
+      if (c->fv && two) {
+        P.fvdiv = c->d_fvdiv + (size_t)(k & 1) * 12 * c->np * half;
+        P.fvdiv_cap = half;
+      }
       P.ebase = (int)ea;
       P.ecount = (int)(eb - ea);
       if (c->mixed)
