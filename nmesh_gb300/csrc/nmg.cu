@@ -2555,7 +2555,7 @@ static int last_step_streamed(nmg_ctx *c, double t, double dt, double *host_u,
         CK(run_stage(c, c->sel, P, ea == 0));  // (not reached: mixed meshes step unstreamed)
       else
         CK(c->variants[c->sel].launch(P, sk));
-      if (!c->mixed) c->launches++;
+      if (!c->mixed) c->launches += variant_launches(c->variants[c->sel], P);
       CK(cudaEventRecord(c->chunk_ev[k], sk));
       CK(cudaStreamWaitEvent(c->copy_stream, c->chunk_ev[k], 0));
       CK(cudaMemcpyAsync(host_u + ea * per, ACC + ea * per, (size_t)(eb - ea) * per * sizeof(double),

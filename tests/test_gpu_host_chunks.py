@@ -50,3 +50,17 @@ def test_finite_volume_mesh(monkeypatch, kind, n, luni, steps, chunks):
 def test_finite_volume_mesh_by_size(steps):
     """3584 elements of 7^3 points: eight chunks by the size rule."""
     _equal(_mesh("shells", 7, 3, fv=True), "", 1e-3, steps, repeats=3)
+
+
+@pytest.mark.parametrize("variant,kernels", [("fvc", 2), ("fvx", 1), ("fv", 1)])
+def test_launches_of_a_chunked_finite_volume_step(monkeypatch, variant, kernels):
+    """Every kernel counts: a chunk of "fvc" is two launches."""
+    monkeypatch.setenv("NMG_COPY_CHUNKS", "8")
+    m = _mesh("box", 5, 2, fv=True)
+    ev = ng.Evolution(m, ng.BC_OUTGOING)
+    ev.set_kernel(variant)
+    u = np.zeros((m.nelem, 5, m.np))
+    before = ev.launches
+    ev.rk4_steps_host(u, 0.0, 1e-3, 1)
+    assert ev.launches - before == (3 + 8) * kernels
+    ev.close()
