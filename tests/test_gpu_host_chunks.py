@@ -64,3 +64,34 @@ def test_launches_of_a_chunked_finite_volume_step(monkeypatch, variant, kernels)
     ev.rk4_steps_host(u, 0.0, 1e-3, 1)
     assert ev.launches - before == (3 + 8) * kernels
     ev.close()
+
+
+DG = [(n, "tc") for n in range(4, 11)] + [(8, "tc:1:256"), (10, "tc:1:256")]
+DG += [(n, "tcl") for n in range(6, 11)] + [(n, "gather:1:128") for n in range(2, 7)]
+DG += [(n, v) for n in (3, 6, 11) for v in ("eo", "gather", "eof")]
+
+
+@pytest.mark.parametrize("chunks", [8, 16])
+@pytest.mark.parametrize("steps", [1, 3])
+@pytest.mark.parametrize("n,variant", DG)
+def test_conforming_mesh(monkeypatch, n, variant, steps, chunks):
+    """A single step starts by element lists of several groups (tcl: two CTAs an entry)."""
+    monkeypatch.setenv("NMG_COPY_CHUNKS", str(chunks))
+    _equal(_mesh("shells", n, 1), variant, 1e-3, steps)
+    _equal(_mesh("box", n, 2), variant, 1e-3, steps)
+
+
+@pytest.mark.parametrize("steps", [1, 3])
+@pytest.mark.parametrize("n,luni", [(9, 3), (6, 3)])
+def test_conforming_mesh_by_size(n, luni, steps):
+    """3584 elements: eight and three chunks by the size rule."""
+    _equal(_mesh("shells", n, luni), "tc", 1e-3, steps)
+
+
+@pytest.mark.parametrize("chunks", [2, 8])
+@pytest.mark.parametrize("steps", [1, 3])
+@pytest.mark.parametrize("n,variant", [(n, v) for n, v in DG if n > 3])
+def test_refined_mesh(monkeypatch, n, variant, steps, chunks):
+    """Non-conforming faces: only the last stage runs in chunks."""
+    monkeypatch.setenv("NMG_COPY_CHUNKS", str(chunks))
+    _equal(_mesh("shells", n, 1, hrefine=(0, 3)), variant, 1e-3, steps)
