@@ -68,12 +68,9 @@ __device__ __forceinline__ void tc_prefetch_l2(const void *p, unsigned bytes) {
                  : "memory");
 }
 
-// 7 signed 8-bit digits of v on the grid of exponent Emax, as fp16 pairs
-__device__ __forceinline__ uint4 tc_digits(double v, int emax) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const int e = (int)(b >> 52) & 0x7FF;
-  const unsigned long long m = e ? ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) : 0ull;
-  const int d = emax - e;  // >= 0
+// signed 8-bit digits, as fp16 pairs, of a significand m on the grid d >= 0 binary
+// places above its own
+__device__ __forceinline__ uint4 tc_split(unsigned long long m, int d, bool neg) {
   const unsigned long long X = d < 64 ? (m << 11) >> d : 0ull;
   const unsigned hi = (unsigned)(X >> 32), lo = (unsigned)X;
   // 0x64dd = fp16 of 1024 + dd (exact); subtracting 1024 leaves the digit
@@ -82,7 +79,6 @@ __device__ __forceinline__ uint4 tc_digits(double v, int emax) {
   h[1] = __byte_perm(hi, 0x64u, 0x4041);
   h[2] = __byte_perm(lo, 0x64u, 0x4243);
   h[3] = __byte_perm(lo, 0x64u, 0x4041);
-  const bool neg = (b >> 63) != 0;
   const __half2 s2 = neg ? __floats2half2_rn(-1.f, -1.f) : __floats2half2_rn(1.f, 1.f);
   const __half2 o2 = neg ? __floats2half2_rn(1024.f, 1024.f) : __floats2half2_rn(-1024.f, -1024.f);
 #pragma unroll
@@ -92,6 +88,13 @@ __device__ __forceinline__ uint4 tc_digits(double v, int emax) {
     h[k] = *reinterpret_cast<uint32_t *>(&x);
   }
   return make_uint4(h[0], h[1], h[2], h[3]);
+}
+
+// the digits of v on the grid of exponent emax (v = 0 below the normal range)
+__device__ __forceinline__ uint4 tc_digits(double v, int emax) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)(b >> 52) & 0x7FF;
+  return tc_split(e ? ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) : 0ull, emax - e, b >> 63);
 }
 
 // T 2^delta as FP64: T converted with one rounding to nearest, then its
