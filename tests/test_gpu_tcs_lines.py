@@ -37,6 +37,16 @@ def _scaled(n, field):
     return u, u * amp, amp
 
 
+def _transposed(m, variant, x):
+    import torch
+    ev = ng.Evolution(m, ng.BC_OUTGOING)
+    ev.set_kernel(variant)
+    rbar, wbar = torch.as_tensor(x).cuda(), torch.empty(x.shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ev.rhs_vjp_device(rbar.data_ptr(), wbar.data_ptr())
+    return wbar.cpu().numpy()
+
+
 @pytest.mark.parametrize("field,out", [(0, 1), (1, 0)])
 @pytest.mark.parametrize("n,variant", CASES + [(n, "eo") for n in (4, 9)])
 def test_every_line_has_its_own_scale(n, variant, field, out):
@@ -51,17 +61,24 @@ def test_every_line_has_its_own_scale(n, variant, field, out):
 @pytest.mark.parametrize("field,out", [(0, 1), (1, 0)])
 @pytest.mark.parametrize("n,variant", VJP + [(4, "vjp"), (9, "vjp")])
 def test_every_transposed_line_has_its_own_scale(n, variant, field, out):
-    import torch
     u, small, amp = _scaled(n, field)
+    assert np.array_equal(_transposed(_box(n), variant, small)[:, out],
+                          _transposed(_box(n), variant, u)[:, out] * amp)
+
+
+@pytest.mark.parametrize("field,out", [(0, 1), (1, 0)])
+@pytest.mark.parametrize("n", [7, 9])
+def test_the_line_left_over_has_its_own_scale(n, field, out):
+    """49 and 81 lines are 3 and 5 tiles and a line, which is an FP64 dot product ("tc" and
+    "tcvjp" at n = 7 and 9; their tiles have one grid per element)."""
+    u, _, _ = _scaled(n, field)
+    small = u.copy()
+    small[:, :, -n:] *= 2.0 ** -40
     ev = ng.Evolution(_box(n), ng.BC_OUTGOING)
-    ev.set_kernel(variant)
-    res = []
-    for x in (u, small):
-        rbar, wbar = torch.as_tensor(x).cuda(), torch.empty(x.shape, dtype=torch.float64, device="cuda")
-        torch.cuda.synchronize()
-        ev.rhs_vjp_device(rbar.data_ptr(), wbar.data_ptr())
-        res.append(wbar.cpu().numpy()[:, out])
-    assert np.array_equal(res[1], res[0] * amp)
+    ev.set_kernel("tc")
+    assert np.array_equal(ev.rhs(small)[:, out, -n:], ev.rhs(u)[:, out, -n:] * 2.0 ** -40)
+    got, want = (_transposed(_box(n), "tcvjp", x)[:, out, -n:] for x in (small, u))
+    assert np.array_equal(got, want * 2.0 ** -40)
 
 
 @pytest.mark.parametrize("n,variant", CASES)
