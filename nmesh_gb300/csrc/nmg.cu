@@ -440,6 +440,14 @@ static unsigned char hang_separable(const nmg_mesh &m, size_t h) {
   return 0;
 }
 
+// Traces between the elements of the two point types: rounded as the finite-volume
+// variant v is, in the reference's order for "fvx"
+static cudaError_t run_ghost(nmg_ctx *c, int v, int nghost, const int *gtab, const double *win,
+                             double *ghost) {
+  return (strcmp(c->variants[v].name, "fvx") ? nmgk::ghost_launch : nmgk::ghost_exact_launch)(
+      nghost, c->n, gtab, c->d_isfv, c->d_gM, win, ghost, c->stream);
+}
+
 // One stage with variant v.  On a mixed DG / finite-volume mesh a stage is
 // three launches: the interpolated interface traces of the stage input, the
 // DG kernel over all elements (writing only the DG ones) and the
@@ -453,8 +461,7 @@ static cudaError_t run_stage(nmg_ctx *c, int v, StageParams P, bool traces = tru
     c->launches++;
   }
   if (c->mixed) {
-    e = nmgk::ghost_launch(c->nghost, c->n, c->d_gtab, c->d_isfv, c->d_gM, P.win, c->d_ghost,
-                           c->stream);
+    e = run_ghost(c, c->fsel, c->nghost, c->d_gtab, P.win, c->d_ghost);
     if (e != cudaSuccess) return e;
     c->launches++;
     // the two kinds of elements side by side: each launch reads the stage input and
@@ -1640,8 +1647,7 @@ static int redo_rhs(nmg_ctx *c, const std::vector<int> &T, const double *w_old,
   if (ng > 0) {
     CK(cudaMemcpyAsync(c->d_gtab2, gtab.data(), sizeof(int) * gtab.size(),
                        cudaMemcpyHostToDevice, c->stream));
-    CK(nmgk::ghost_launch(ng, c->n, c->d_gtab2, c->d_isfv, c->d_gM, w_old, c->d_ghost2,
-                          c->stream));
+    CK(run_ghost(c, c->fsel >= 0 ? c->fsel : fv_default(c), ng, c->d_gtab2, w_old, c->d_ghost2));
     c->launches++;
   }
   StageParams Q = base_params(c);

@@ -642,6 +642,10 @@ cudaError_t hang_adj_launch(int nhang, int n, const int *toff, const int *tsrc, 
                             cudaStream_t st);
 cudaError_t ghost_launch(int nghost, int n, const int *gtab, const unsigned char *isfv,
                          const double *M, const double *win, double *ghost, cudaStream_t st);
+// the same rounded in the reference's order (for "fvx"; stage_fv.cu)
+cudaError_t ghost_exact_launch(int nghost, int n, const int *gtab, const unsigned char *isfv,
+                               const double *M, const double *win, double *ghost,
+                               cudaStream_t st);
 // u of the listed elements <- (M x M x M) u (all fields), in place
 cudaError_t convert_launch(int n, const int *list, int count, const double *M, double *u,
                            cudaStream_t st);

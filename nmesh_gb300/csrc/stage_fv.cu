@@ -444,6 +444,36 @@ int fv_variants(int n, Variant *out, int cap) {
 }
 
 namespace {
+// The traces between elements of the two point types beside "fvx", whose elements are
+// rounded in the reference's order throughout: sum_k sum_j v(j, k) B1[j] B2[k], one product
+// and sum at a time (basis_array_interp2d, src/main/basis/interpolate.c:296; this file
+// has no FMA contraction).  One thread per (slot, field, face node).
+__global__ void __launch_bounds__(256) ghost_exact_kernel(int nghost, int n, const int *gtab,
+                                                         const unsigned char *isfv,
+                                                         const double *M, const double *win,
+                                                         double *ghost) {
+  const int nn = n * n, np = nn * n;
+  const int64_t total = (int64_t)nghost * 4 * nn;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    const int g = (int)(q / (4 * nn)), rem = (int)(q - (int64_t)g * 4 * nn);
+    const int l = rem / nn, ab = rem - l * nn, a = ab % n, b = ab / n;
+    const int e2 = __ldg(gtab + 4 * g + 2), cd = __ldg(gtab + 4 * g + 3), o = (cd >> 3) & 7;
+    int aa = (o & 1) ? b : a, bb = (o & 1) ? a : b;
+    if (o & 2) aa = n - 1 - aa;
+    if (o & 4) bb = n - 1 - bb;
+    const double *Mk = M + (isfv[e2] ? nn : 0);
+    const double *v = win + ((size_t)e2 * NF + l) * np;
+    double sum = 0.;
+    for (int k = 0; k < n; k++) {
+      const double B2 = __ldg(Mk + bb * n + k);
+      for (int j = 0; j < n; j++)
+        sum += __ldg(v + fv_exact::fnode(n, cd & 7, j, k)) * __ldg(Mk + aa * n + j) * B2;
+    }
+    ghost[(size_t)g * 4 * nn + l * nn + ab] = sum;
+  }
+}
+
 // Transpose of the non-conforming traces for the adjoint: the neighbour part
 // of a face lift (g d pi + gn . d c, gn d pi + g d c) on slot h's face, with
 // d the trace, becomes, per field, the adjoint tb = (g rbar_pi + gn . rbar_c,
@@ -495,6 +525,16 @@ __global__ void __launch_bounds__(256) hang_adj_kernel(int nhang, int n, const i
   }
 }
 }  // namespace
+
+cudaError_t ghost_exact_launch(int nghost, int n, const int *gtab, const unsigned char *isfv,
+                               const double *M, const double *win, double *ghost,
+                               cudaStream_t st) {
+  if (nghost <= 0) return cudaSuccess;
+  const int64_t total = (int64_t)nghost * 4 * n * n;
+  const int grid = (int)std::min<int64_t>((total + 255) / 256, 152 * 16);
+  ghost_exact_kernel<<<grid, 256, 0, st>>>(nghost, n, gtab, isfv, M, win, ghost);
+  return cudaGetLastError();
+}
 
 cudaError_t hang_adj_launch(int nhang, int n, const int *toff, const int *tsrc, const double *tw,
                             const int *hface, const int *cslot, const double *fac,
