@@ -979,6 +979,25 @@ static void drop_graphs(nmg_ctx *c) {
 
 extern "C" {
 
+// scratch of the "fvc" kernels for nfv finite-volume elements (in groups, so that a
+// smaller one will do where there is no memory)
+static int grow_fvdiv(nmg_ctx *c, int nfv) {
+  const int cap = nmgk::fvc_capacity(c->n, nfv);
+  if (cap <= c->fvdiv_cap) return NMG_OK;
+  double *d = nullptr;
+  if (cudaMalloc((void **)&d, sizeof(double) * 12 * c->np * cap) != cudaSuccess) {
+    cudaGetLastError();
+    if (c->fvdiv_cap > 0) return NMG_OK;
+    return set_err(c, NMG_ENOMEM, "finite-volume scratch: device allocation failed");
+  }
+  CK(cudaStreamSynchronize(c->stream));
+  cudaFree(c->d_fvdiv);
+  drop_graphs(c);
+  c->d_fvdiv = d;
+  c->fvdiv_cap = cap;
+  return NMG_OK;
+}
+
 // Type-dependent tables of a context with finite-volume elements: element
 // flags and list, face codes with the mixed bit, interface-trace slots.
 // Rebuilt and uploaded whenever element types change.
@@ -1003,15 +1022,7 @@ static int upload_type_tables(nmg_ctx *c) {
     }
   }
   c->nfvel = (int)fvlist.size();
-  // a switchable context may redo a step with more finite-volume elements
-  const int cap = nmgk::fvc_capacity(c->n, c->switchable ? (int)E : c->nfvel);
-  if (cap > c->fvdiv_cap) {
-    cudaFree(c->d_fvdiv);
-    c->d_fvdiv = nullptr;
-    c->fvdiv_cap = 0;
-    CK(cudaMalloc((void **)&c->d_fvdiv, sizeof(double) * 12 * c->np * cap));
-    c->fvdiv_cap = cap;
-  }
+  if (int rc = grow_fvdiv(c, c->nfvel)) return rc;
   c->nghost = (int)(gtab.size() / 4);
   if (c->nghost > c->ghost_cap) {
     cudaFree(c->d_ghost);
@@ -1650,6 +1661,7 @@ static int redo_rhs(nmg_ctx *c, const std::vector<int> &T, const double *w_old,
     CK(run_ghost(c, c->fsel >= 0 ? c->fsel : fv_default(c), ng, c->d_gtab2, w_old, c->d_ghost2));
     c->launches++;
   }
+  if (int rc = grow_fvdiv(c, (int)T.size())) return rc;
   StageParams Q = base_params(c);
   Q.win = w_new;
   Q.mode = 0;
