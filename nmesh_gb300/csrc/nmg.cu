@@ -1106,9 +1106,10 @@ static int create_impl(const nmg_mesh *m, int32_t bc_kind, const double k[3], bo
       return set_err(c, NMG_EUNSUP, "nmg_create: no transposed kernel for this n");
     c->nvjp_alt = 1 + nmgk::tcvjp_variants(m->n, &c->vjp_alt[1], 1);
     c->nvjp_alt += nmgk::tcsv_variants(m->n, &c->vjp_alt[c->nvjp_alt], 3 - c->nvjp_alt);
-    // "tcvjp" where there are tensor-core forms, on meshes of few elements "tcvjw" where
-    // there is that one, else "vjp"
-    const char *want = m->nelem <= nmgk::tcvjw_elements(m->n) ? "tcvjw" : "tcvjp";
+    int vdev = 0, sms = 0;
+    CK(cudaGetDevice(&vdev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, vdev));
+    const char *want = nmgk::vjp_choice(m->n, m->nelem, sms);
     c->vjp = c->vjp_alt[0];
     for (int v = 1; v < c->nvjp_alt; v++)
       if (!strcmp(c->vjp_alt[v].name, want)) c->vjp = c->vjp_alt[v];

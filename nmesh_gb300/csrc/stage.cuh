@@ -579,8 +579,9 @@ int tcs_variants(int n, Variant *out, int cap);
 cudaError_t tcs_upload(int n, const double *D);
 // transposed stage: "tcvjp" for n = 4, 5, 6, 10 and "tcvjw", its form for few elements
 int tcsv_variants(int n, Variant *out, int cap);
-// up to as many elements "tcvjw" (at n = 6 the FP64 kernel) is the faster one
-int64_t tcvjw_elements(int n);
+// the transposed kernel of a mesh: on meshes whose elements fit the sms SMs at once in
+// "tcvjw" that one (at n = 6 "vjp"), else "tcvjp", and "vjp" where those are not compiled
+const char *vjp_choice(int n, int64_t nelem, int sms);
 // tensor-core transposed (vector-Jacobian) stage kernel for n = 7, 8, 9
 int tcvjp_variants(int n, Variant *out, int cap);
 // transposed (vector-Jacobian) stage kernel for n

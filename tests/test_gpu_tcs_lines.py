@@ -40,7 +40,8 @@ def _scaled(n, field):
 def _transposed(m, variant, x):
     import torch
     ev = ng.Evolution(m, ng.BC_OUTGOING)
-    ev.set_kernel(variant)
+    if variant:
+        ev.set_kernel(variant)
     rbar, wbar = torch.as_tensor(x).cuda(), torch.empty(x.shape, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     ev.rhs_vjp_device(rbar.data_ptr(), wbar.data_ptr())
@@ -110,3 +111,16 @@ def test_values_below_the_normal_range(n, variant):
     assert np.abs(r[0]).max() > 1000 * 2.0 ** -1074
     # three directions of n products, six faces of four terms
     assert np.abs(r[0] - r[1]).max() / 2.0 ** -1074 <= 3 * (n + 2) + 24
+
+
+@pytest.mark.parametrize("n,few,many", [(6, "vjp", "tcvjp"), (7, "tcvjw", "tcvjp"), (9, "tcvjw", "tcvjp"),
+                                        (11, "vjp", "vjp")])
+def test_choice_of_the_transposed_kernel(n, few, many):
+    """By the number of SMs: 64 elements have room at once, 4096 have not (the kernels differ
+    in their last bits)."""
+    for luni, name in ((2, few), (4, many)):
+        m = ng.Mesh.build(ng.MESH_BOX, n=n, luni=luni, xc=(PI, PI, PI), box_dout=PI, periodic=True)
+        x = np.random.default_rng(n).standard_normal((m.nelem, 5, m.np))
+        got = _transposed(m, None, x)
+        for k in {"vjp", few, many}:
+            assert np.array_equal(got, _transposed(m, k, x)) == (k == name), (luni, k)
