@@ -264,6 +264,7 @@ struct nmg_ctx {
   // stages read the step's time on the device: exact outer faces.  Without them a
   // step is its stages alone (512 elements at n = 5: 67.9 -> 64.6 us a step)
   bool timed = false;
+  bool digits8 = false;  // eight digits at n = 7 and 9 too (tune_skips)
   double k[3] = {0, 0, 0};
   cudaStream_t stream = nullptr;
   Variant variants[kMaxVariants];
@@ -607,8 +608,17 @@ static StageParams base_params(nmg_ctx *c) {
 // * "fv", "fvx": 1.5 and 2 times the FP64 instructions of "fvc" for the same work;
 // * "eof", "eofu": at best within 1 % of "eo" (n = 8, 12), else 1.05 to 2 times it;
 // * "eo" with 128 threads, or with the elements of two tiles in a CTA.
+// And at n = 7 and 9 one of the two digit-product kernels: "tc", with seven digits on one
+// grid per element, has up to 1.7 times the FP64 kernels' error (56 elements of the cubed
+// spheres, n = 9: 3.1e-15 against 1.8e-15; a box at n = 7: 1.07e-15 against 0.83 to 0.89), "tc8"
+// (eight on a grid per line, stage_tcs.cu) theirs.  "tc" is for meshes of DG elements of one
+// order, where it is the faster one (7 x 8^3 elements, n = 9 374 against 396 us, n = 7 186 against
+// 207), "tc8" (digits8) for the others: orders in a batch, DG beside finite volume at
+// n = 7, a box at n = 7 (16^3 elements 166 against 172 us, 8^3 33 against 31).
 static bool tune_skips(const nmg_ctx *c, int v) {
   const nmgk::Variant &k = c->variants[v];
+  if (!strcmp(k.name, "tc8")) return !c->digits8;
+  if (!strcmp(k.name, "tc") && (c->n == 7 || c->n == 9)) return c->digits8;
   if (!strncmp(k.name, "fv", 2)) return strcmp(k.name, "fvc") != 0;
   if (!strncmp(k.name, "eof", 3)) return true;
   if (strcmp(k.name, "eo")) return false;
@@ -639,7 +649,8 @@ static int tune_range(nmg_ctx *c, int v0, int v1, bool fvpart, int *best_out) {
   std::vector<int> order;
   for (int tc = 1; tc >= 0; tc--)
     for (int v = v0; v < v1; v++)
-      if ((strcmp(c->variants[v].name, "tc") == 0) == (tc == 1) && !tune_skips(c, v))
+      if ((!strcmp(c->variants[v].name, "tc") || !strcmp(c->variants[v].name, "tc8")) == (tc == 1) &&
+          !tune_skips(c, v))
         order.push_back(v);
   for (int v : order) {
     StageParams P = base_params(c);
@@ -1149,6 +1160,7 @@ static int create_impl(const nmg_mesh *m, int32_t bc_kind, const double k[3], bo
   }
   // (a mixed mesh, with three long launches or more a stage, keeps its step counter)
   c->timed = (bc_kind == NMG_BC_EXACT_PLANEWAVE && B > 0) || c->mixed;
+  c->digits8 = m->n == 7 && (c->mixed || C == 0);
   c->ncurvi = C;
   c->nbface = B;
   c->h_cslot = cslot;
@@ -3173,6 +3185,7 @@ static int batch_create_impl(const nmg_mesh *const *meshes, int32_t count, const
     b->gmesh.push_back(mm);
     nmg_ctx *c = nullptr;
     int rc = nmg_create(mm, bc_kind, k, &c);
+    if (c) c->digits8 = c->n == 7 || c->n == 9;
     b->gctx.push_back(c);
     if (rc) return batch_err(b, rc, std::string("nmg_batch_create: ") + nmg_last_error(c));
     b->gn.push_back(n);
