@@ -198,7 +198,7 @@ def fp64_variant_line(kinfo, nelem, ncurvi, n, fp64_peak):
             "issue_frac": ins / (ms / 1e3) / (fp64_peak * 1e9 / 2),
             "note": "the selected tensor-core kernel issues ~40 % fewer FP64 "
                     "instructions and is latency-bound (ncu: FP64 pipe 63 % busy, tensor "
-                    "pipe ~13 %, profiles/tc_kernel_n9_cubedspheres_l3_stage1.md); its "
+                    "pipe ~13 % at level 3); its "
                     "roofline_fp64 counts only its own FP64 work"}
 
 
@@ -731,9 +731,8 @@ def fv_bench(args):
                             "flops_per_launch_model": flops,
                             "peak_source": "FP64 FMA probe run live (nmg_fp64_peak)",
                             "note": "the model counts the operations of the per-midpoint form "
-                                    "(\"fv\"), of which \"fvc\" needs fewer; the FP64 pipe "
-                                    "utilization from ncu is in "
-                                    "profiles/fvc_kernel_n13_cubedspheres_l2_rhs.md"}
+                                    "(\"fv\"), of which \"fvc\" needs fewer (ncu: FP64 pipe "
+                                    "85.5 % busy at level 2)"}
     if not args.no_cpu_baseline:
         cl = args.fv_cpu_luni
         cxyz, om = cpu_mesh(n, cl, fv=True, fv_rec=rec, fv_extrap=ex)

@@ -176,7 +176,9 @@ const char *nmg_mesh_last_error(void);
 
 /* ---- device context ----------------------------------------------------- */
 /* Uploads the mesh (metric, face factors, face table) and allocates the RK4
- * state (u, u accumulator, two stage buffers) on the current CUDA device.
+ * state (u, u accumulator, two stage buffers) on the current CUDA device; with
+ * finite-volume elements also a scratch of 96 bytes for each of their points, at
+ * most 256 MB.
  * bc_kind: NMG_BC_*; k: plane-wave vector for NMG_BC_EXACT_PLANEWAVE. */
 int nmg_create(const nmg_mesh *m, int32_t bc_kind, const double k[3],
                nmg_ctx **out);
@@ -353,7 +355,9 @@ int nmg_grhd_sizes(const nmg_grhd_ctx *c, int32_t *n, int32_t *nf, int64_t *nele
 /* element modes (fv[e] = 1: finite volume) with the state transferred
  * (trouble.c:162-183, gridpoints.c:158-200): to finite volume by Lagrange
  * interpolation P from the LGL points to the nf equally spaced points in
- * each direction, back by the pseudo-inverse R = (P^T P)^-1 P^T */
+ * each direction, back by the pseudo-inverse R = (P^T P)^-1 P^T.  A point of a
+ * finite-volume element takes 632 bytes on the device: four states, the
+ * primitives, the geometry and the three directions' flux differences */
 int nmg_grhd_set_fv_elements(nmg_grhd_ctx *c, const int32_t *fv);
 int nmg_grhd_get_fv_elements(nmg_grhd_ctx *c, int32_t *fv);
 /* Persson's modal indicator of D per element (evolve_Persson_array_indicator,
@@ -479,7 +483,8 @@ int nmg_rk4_steps_host(nmg_ctx *c, double t, double dt, int32_t nsteps,
  * the same order are merged into one mesh (nmg_mesh_concat); one persistent
  * kernel launch per RK4 stage walks the element tiles of all orders
  * (runtime dispatch to the order's kernel body, highest order first), and
- * one RK4 step (4 launches + a step counter) is captured in a CUDA graph.
+ * one RK4 step (4 launches, and a step counter with exact outer faces) is
+ * captured in a CUDA graph.
  * The persistent grid size is chosen by timing (autotuner).  All problems
  * share t, dt and the boundary kind. */
 typedef struct nmg_batch nmg_batch;
@@ -559,7 +564,8 @@ int nmg_rk4_step_noalloc(nmg_ctx *c, double t, double dt, const double *u_in_dev
  * stage kernel ("eo": even-odd line derivatives, "gather": node-parallel dot
  * products, "tc" at n = 4, ..., 10: line derivatives on the tensor cores as
  * exact integer digit products, "tcl" at n = 6, ..., 10: the form of it for few
- * elements; "eof"/"eofu", with the face lift in the line passes, run when asked
+ * elements, "tc8" at n = 7, 9: with the accuracy of the FP64 kernels, in the place of
+ * "tc" for the orders of a batch and at n = 7 on mixed meshes and boxes; "eof"/"eofu", with the face lift in the line passes, run when asked
  * for) and tile shapes (elements and threads per CTA) on the context's mesh and
  * keeps the fastest.  spec = "auto" re-tunes; a name such as "eo",
  * "gather" or "tc", or "<name>:<elements per CTA>:<threads>", forces a

@@ -360,7 +360,8 @@ __device__ __forceinline__ void update_batch(const StageParams &P, int e, int q0
       if (KEEP && k0 + j < NK) keep[k0 + j] = wi[j];
     }
     // never taken (the kernels return for such elements): without a branch here the
-    // loads are ordered otherwise, and n = 6 is 1 %, an ensemble of orders 3.5 % slower
+    // loads are ordered otherwise, and a stage is slower (7 x 8^3 elements, n = 8 221 -> 227
+    // us, n = 6 126.8 -> 128.3, n = 5 81.8 -> 83.0; the others within 0.5 %)
     if (P.skip && P.skip[e]) continue;
 #pragma unroll
     for (int j = 0; j < NB; j++) {
@@ -574,7 +575,8 @@ int eo_variants(int n, Variant *out, int cap);
 int tc_variants(int n, Variant *out, int cap);
 // digits of D and D^T for the tensor-core variants (no-op for other n)
 cudaError_t tc_upload(int n, const double *D);
-// the same for n = 4, 5, 6, 8, 10, and for meshes of few elements, n = 6 to 10 (stage_tcs.cu)
+// the same for n = 4, 5, 6, 8, 10 ("tc8" at n = 7, 9), and for meshes of few elements,
+// n = 6 to 10 (stage_tcs.cu)
 int tcs_variants(int n, Variant *out, int cap);
 cudaError_t tcs_upload(int n, const double *D);
 // transposed stage: "tcvjp" for n = 4, 5, 6, 10 and "tcvjw", its form for few elements
